@@ -285,7 +285,7 @@ struct b200_decoder {
     std::map<std::pair<int, double>, float2*> rot_tables;
     std::vector<Slot> slots;
     // activations of the general path
-    float *x = nullptr, *proj = nullptr, *y = nullptr, *aux = nullptr, *wide = nullptr;
+    float *x = nullptr, *proj = nullptr, *y = nullptr, *aux = nullptr, *wide = nullptr, *chunks = nullptr;
     void *h = nullptr, *conv = nullptr, *mix = nullptr, *q = nullptr, *low = nullptr;
     float *gates = nullptr;                          // low-rank decays and output gates
     void *ql = nullptr, *lat = nullptr, *kv = nullptr;  // latent queries; latents and expanded keys and values of the step (grown on demand)
@@ -750,7 +750,7 @@ void load_all(b200_decoder* m) {
 
 // activations, sized from the loaded layers
 void allocate(b200_decoder* m) {
-    size_t proj = 0, mix = 0, conv = 0, aux = 0, wide = 0, q = 0, low = 0, gates = 0, ql = 0, raw = 0, decode_pair_mix = 0, top = 0;
+    size_t proj = 0, mix = 0, conv = 0, aux = 0, wide = 0, q = 0, low = 0, gates = 0, ql = 0, raw = 0, decode_pair_mix = 0, top = 0, chunks = 0;
     size_t pair_rows = 0, pair_mix = 0;  // (pair_mix, raw: elements)
     bool shared = false;
     auto up = [](size_t& a, size_t b) { if (b > a) a = b; };
@@ -762,7 +762,7 @@ void allocate(b200_decoder* m) {
         switch (s.kind) {
             case MIX_MAMBA1: up(conv, L.np); up(aux, L.xp.N); up(wide, L.np); up(low, L.rank_p); break;
             case MIX_CHANNEL_DELTA: up(low, L.low.K); up(gates, L.low.N);  // and
-            case MIX_DELTA: up(conv, 2 * L.np); up(wide, s.heads * L.Dvl); up(aux, 4 * s.heads); break;  // (fp32 in either arithmetic)
+            case MIX_DELTA: up(conv, 2 * L.np); up(wide, s.heads * L.Dvl); up(aux, 2 * s.heads); up(chunks, delta_chunk_floats(m->max_rows, m->max_slots, s.heads)); break;  // (fp32 in either arithmetic)
             case MIX_PARALLEL: up(q, (size_t)L.att.H * L.att.Dp); break;
             case MIX_LATENT:
                 up(q, (size_t)L.lat.H * L.lat.Dp);
@@ -791,6 +791,7 @@ void allocate(b200_decoder* m) {
     m->conv = device_zeros(m, M * conv * (m->f32 ? 4 : 2));
     m->aux = static_cast<float*>(device_zeros(m, M * aux * 4));
     m->wide = static_cast<float*>(device_zeros(m, M * wide * 4));
+    m->chunks = static_cast<float*>(device_zeros(m, chunks * 4));
     m->low = device_zeros(m, M * low * e);
     m->q = device_zeros(m, M * q * e);
     m->gates = static_cast<float*>(device_zeros(m, M * gates * 4));
@@ -981,11 +982,12 @@ int mixer_delta(b200_decoder* m, const Layer& L, const StepView& v) {
     DeltaArgs a = delta_args(m, L, v.seqs, m->proj);
     a.qkv = static_cast<const float*>(m->conv);
     a.raw = m->proj; a.ld_raw = L.in.N;
-    a.coef = reinterpret_cast<float4*>(m->aux);
+    a.coef = reinterpret_cast<float2*>(m->aux);
+    a.chunks = m->chunks;
     if (channel) { a.decay = m->gates; a.ld_decay = L.low.N; }
     OP("delta prep", launch_delta_prep(ctx, a, v.E, v.max_n));
     a.out = m->wide; a.ldo = s.heads * L.Dvl;
-    OP("delta scan", launch_delta_scan(ctx, a, v.E));
+    OP("delta scan", launch_delta_scan(ctx, a, v.E, v.max_n));
     OP("head norm", launch_gated_head_norm(ctx, m->mix, L.o.K, m->wide, a.ldo, channel ? m->gates + L.gate_row : m->proj + L.gate_col, channel ? L.low.N : L.in.N,
                                            L.head_norm, v.M, s.heads, s.vdim, L.Dvl, m->spec.eps, m->f32, channel));
     return B200_OK;

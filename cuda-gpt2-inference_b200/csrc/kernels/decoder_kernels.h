@@ -135,13 +135,14 @@ int launch_selective_scan(b200_ctx* ctx, const SelectiveScanArgs& a, int E, int 
 // State [slots][H][Dv][Dpad] fp32.
 //   prep   convolution + silu of raw's q and k columns -> unit vectors (q also times D^-1/2) in qkv, and coef
 //          (the v columns are a plain short convolution)
-//   scan   qkv, coef -> o in out [M, H*Dvl] fp32
+//   scan   qkv, coef (16 tokens at a time) -> o in out [M, H*Dvl] fp32
 //   step   one token per sequence, from the convolved columns (qkv, ld) to the normalised, gated output as split rows
 //          of ldo columns
 struct DeltaArgs {
     const float* qkv; int ld; int k_col, v_col;
     const float* raw; int ld_raw;
-    float4* coef;           // [M][H] {decay, beta, k.q, -}
+    float2* coef;           // [M][H] {decay, beta}
+    float* chunks;          // scan: delta_chunk_floats() of workspace
     const float* gates; int ldg; int a_col, b_col;  // columns of the projection holding a and b per head
     const float* negA;      // [H] -exp(A_log)
     const float* dt_bias;   // [H]
@@ -160,7 +161,8 @@ struct DeltaArgs {
 };
 int delta_state_pad(int D);  // 0: unsupported
 int launch_delta_prep(b200_ctx* ctx, const DeltaArgs& a, int E, int max_n);
-int launch_delta_scan(b200_ctx* ctx, const DeltaArgs& a, int E);
+int launch_delta_scan(b200_ctx* ctx, const DeltaArgs& a, int E, int max_n);  // two launches
+size_t delta_chunk_floats(int M, int E, int H);  // of a step of up to M rows in up to E sequences
 int launch_delta_step(b200_ctx* ctx, const DeltaArgs& a, int E);
 
 // minGRU: z = sigmoid(zx[z_col ..]), u = zx[x_col ..], candidate = u + 1/2 (u >= 0) or sigmoid(u);

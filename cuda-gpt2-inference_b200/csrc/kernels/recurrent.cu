@@ -346,7 +346,7 @@ struct DeltaCore {
 };
 
 // What the scan wants per token: convolved and activated q and k as unit vectors (q also times D^-1/2) and, per
-// head, {decay, beta, k.q}.  One warp per (sequence, key/value head, run of 16 tokens), a lane holding channels
+// head, {decay, beta}.  One warp per (sequence, key/value head, run of 16 tokens), a lane holding channels
 // lane, lane + 32, ... (V of them) of q and k; two tokens at a time.
 template <int TAPS, int V>
 __global__ void __launch_bounds__(128)
@@ -390,7 +390,7 @@ delta_prep_kernel(const DeltaArgs a) {
         const int t = t0 + i / per, h = g * per + i % per;
         const float* gr = a.gates + (size_t)(sd.row0 + t) * a.ldg;
         const float decay = a.decay ? 1.f : expf(__ldg(a.negA + h) * softplusf_(gr[a.a_col + h] + __ldg(a.dt_bias + h)));
-        *reinterpret_cast<float2*>(a.coef + (size_t)(sd.row0 + t) * a.H + h) = make_float2(decay, sigmoidf_(gr[a.b_col + h]));
+        a.coef[(size_t)(sd.row0 + t) * a.H + h] = make_float2(decay, sigmoidf_(gr[a.b_col + h]));
     }
     float w[2][V][W], win[2][V][W];  // weights and the window of earlier inputs
     if (TAPS > 0) {
@@ -423,10 +423,10 @@ delta_prep_kernel(const DeltaArgs a) {
                                 in[u][x][i] = fmaf(input(tb + u - hrows + j, base[x] + d), __ldg(a.conv_w + (size_t)j * a.np + base[x] + d), in[u][x][i]);
                     }
                 }
-        float sum[2][3];
+        float sum[2][2];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
-            sum[u][0] = sum[u][1] = sum[u][2] = 0.f;
+            sum[u][0] = sum[u][1] = 0.f;
 #pragma unroll
             for (int i = 0; i < V; ++i) {
 #pragma unroll
@@ -444,7 +444,6 @@ delta_prep_kernel(const DeltaArgs a) {
                 }
                 sum[u][0] = fmaf(in[u][0][i], in[u][0][i], sum[u][0]);
                 sum[u][1] = fmaf(in[u][1][i], in[u][1][i], sum[u][1]);
-                sum[u][2] = fmaf(in[u][0][i], in[u][1][i], sum[u][2]);
             }
         }
 #pragma unroll
@@ -452,7 +451,7 @@ delta_prep_kernel(const DeltaArgs a) {
 #pragma unroll
             for (int u = 0; u < 2; ++u)
 #pragma unroll
-                for (int x = 0; x < 3; ++x) sum[u][x] += __shfl_xor_sync(0xffffffffu, sum[u][x], s);
+                for (int x = 0; x < 2; ++x) sum[u][x] += __shfl_xor_sync(0xffffffffu, sum[u][x], s);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int t = tb + u;
@@ -464,8 +463,6 @@ delta_prep_kernel(const DeltaArgs a) {
 #pragma unroll
                 for (int i = 0; i < V; ++i)
                     if (lane + i * 32 < a.Dl) row[base[x] + lane + i * 32] = in[u][x][i] * r[x];
-            const float kq = sum[u][2] * r[0] * r[1];
-            for (int j = lane; j < per; j += 32) a.coef[(size_t)(sd.row0 + t) * a.H + g * per + j].z = kq;
         }
     }
     if (t1 == sd.n)  // the last inputs are the history of the next step
@@ -476,89 +473,381 @@ delta_prep_kernel(const DeltaArgs a) {
             }
 }
 
-// Prefill: a CTA walks one (sequence, head) for blockDim.x / L * NC columns of Dv, in tiles of 16 tokens (8 with a decay
-// per channel) staged two deep by asynchronous copies.
-__host__ __device__ constexpr int delta_tile_tokens(bool channel) { return channel ? 8 : kDeltaTok; }
-// floats of a tile: q, k, decays, v, coefficients
-__host__ __device__ constexpr int delta_tile_floats(int D, int cpad, bool channel) { return delta_tile_tokens(channel) * ((channel ? 3 : 2) * D + cpad + 4); }
-template <int L, int NC, bool CH>
+// Prefill takes the tokens in chunks of kChunk = 16.  With S the state before a chunk, p_t the product of the decays of its tokens up
+// to and including t, and p_t / p_j short for the product of those behind j,
+//   u_t = beta_t (v_t - S^T (p_t k_t) - sum_{j<t} A_tj u_j),   A_tj = k_t . (p_t / p_j) k_j
+//   o_t = S^T (p_t q_t) + sum_{j<=t} Q_tj u_j,                 Q_tj = q_t . (p_t / p_j) k_j
+//   S  <- p_last S + sum_t ((p_last / p_t) k_t) u_t^T
+// - the token-by-token rule with u solved for: (I + beta A) U = beta R, R = V - (p k) S, so U = T R with T = (I + beta A)^-1 beta.  A, Q
+// and T do not depend on S and come from a kernel that runs over all chunks at once; what is left in the chain from chunk to
+// chunk is three products with the state, which need no reduction per token.  All of it is fp32, every quotient p_t / p_j
+// is formed as a product of decays (none is ever divided by), and T's entries are entries of products of contractions.
+constexpr int kChunk = 16;
+constexpr int kChunkLd = kChunk + 4;                 // rows of T and Q: eight of them in different banks
+constexpr int kChunkFloats = 2 * kChunk * kChunkLd;  // T and Q of a (chunk, head)
+// a sequence's first chunk among those of the step (at most rows / 16 + sequences in all)
+__device__ __forceinline__ float* chunk_matrices(const DeltaArgs& a, const SeqDesc& sd, int seq, int chunk, int h) {
+    return a.chunks + ((size_t)(sd.row0 / kChunk + seq + chunk) * a.H + h) * kChunkFloats;
+}
+
+// T and Q of one (head, chunk, sequence).  Sixteen lanes share the dimensions; a thread's half-warp forms columns jp and 15 - jp
+// (17 pairs in either case), walking the tokens upward with k_j decayed along.
+template <int L, bool CH>
 __global__ void __launch_bounds__(128)
-delta_scan_kernel(const DeltaArgs a) {
-    using Core = DeltaCore<L, NC, CH>;
-    constexpr int D = 16 * L, TOK = delta_tile_tokens(CH), VECS = CH ? 3 : 2;
-    extern __shared__ __align__(16) float sm[];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int cols = blockDim.x / L * NC;
-    const int cpad = (cols + 3) & ~3;
-    const int tile_f = delta_tile_floats(D, cpad, CH);
-    const int h = blockIdx.x, c0 = blockIdx.y * cols;
-    const int kvh = h / (a.H / a.G);
-    // rows of k and q beyond the head's dimension and columns beyond Dv stay zero in both tiles
-    for (int i = tid; i < 2 * tile_f + D; i += blockDim.x) sm[i] = 0.f;
+delta_chunk_kernel(const DeltaArgs a) {
+    constexpr int D = 16 * L, VECS = CH ? 3 : 2, LD = D + 4, NI = L >= 4 ? L / 4 : 1;
+    extern __shared__ __align__(16) float rows[];  // [VECS][kChunk][LD]: q, k, decays
+    __shared__ __align__(16) float A[kChunk * kChunkLd], Q[kChunk * kChunkLd];
+    __shared__ float2 coef[kChunk];
     griddep_wait();
     griddep_launch_dependents();
     const SeqDesc sd = a.seqs[blockIdx.z];
-    const int grp = tid / L, l = tid & (L - 1);
-    const int gc = c0 + grp * NC;           // first column of this group
-    const int ncol = min(NC, a.Dv - gc);    // may be <= 0
+    const int t0 = blockIdx.y * kChunk, h = blockIdx.x, tid = threadIdx.x;
+    if (t0 >= sd.n) return;
+    const int nt = min(kChunk, sd.n - t0), kvh = h / (a.H / a.G), d4 = a.Dl >> 2;
+    const float* src = a.qkv + (size_t)(sd.row0 + t0) * a.ld + kvh * a.Dl;
+    for (int i = tid; i < VECS * kChunk * (D / 4); i += 128) {
+        const int v = i / (kChunk * (D / 4)), t = i / (D / 4) % kChunk, c = i % (D / 4);
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (t < nt && c < d4) {
+            if (v < 2) x = load4(src + (size_t)t * a.ld + (v ? a.k_col : 0), c);
+            else x = load4(a.decay + (size_t)(sd.row0 + t0 + t) * a.ld_decay + (size_t)h * a.Dl, c);
+        }
+        *reinterpret_cast<float4*>(rows + (v * kChunk + t) * LD + c * 4) = x;
+    }
+    if (tid < kChunk) coef[tid] = tid < nt ? a.coef[(size_t)(sd.row0 + t0 + tid) * a.H + h] : make_float2(1.f, 0.f);
+    for (int i = tid; i < kChunk * kChunkLd; i += 128) A[i] = Q[i] = 0.f;
+    __syncthreads();
+    const int s = tid & 15, jp = tid >> 4;
+    const bool live = s * 4 < D;
+    const int j[2] = {jp, kChunk - 1 - jp};
+    float4 kj[2][NI];
+    float decayed[2] = {1.f, 1.f};
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            kj[x][i] = live ? *reinterpret_cast<const float4*>(rows + (kChunk + j[x]) * LD + s * 4 + 64 * i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    auto dot = [](const float4& x, const float4& y, float c) { return fmaf(x.x, y.x, fmaf(x.y, y.y, fmaf(x.z, y.z, fmaf(x.w, y.w, c)))); };
+    // (the two halves of a warp have neighbouring jp: they start together)
+#pragma unroll 4
+    for (int t = jp & ~1; t < nt; ++t) {
+        float sum[4] = {0.f, 0.f, 0.f, 0.f};  // A, Q of column j[0], of column j[1]
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const float* p = rows + t * LD + s * 4 + 64 * i;
+            const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+            const float4 q = live ? *reinterpret_cast<const float4*>(p) : zero, k = live ? *reinterpret_cast<const float4*>(p + kChunk * LD) : zero;
+            const float4 g = CH && live ? *reinterpret_cast<const float4*>(p + 2 * kChunk * LD) : zero;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                if (CH && t > j[x]) { kj[x][i].x *= g.x; kj[x][i].y *= g.y; kj[x][i].z *= g.z; kj[x][i].w *= g.w; }
+                sum[2 * x] = dot(k, kj[x][i], sum[2 * x]);
+                sum[2 * x + 1] = dot(q, kj[x][i], sum[2 * x + 1]);
+            }
+        }
+        if (!CH) {
+            const float g = coef[t].x;
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                if (t > j[x]) decayed[x] *= g;
+                sum[2 * x] *= decayed[x];
+                sum[2 * x + 1] *= decayed[x];
+            }
+        }
+        reduce_scatter<4, 16>(sum, tid & 31);
+        const int which = scatter_first<4, 16>(tid & 31), col = j[which >> 1];
+        if (scatter_owner<4, 16>(tid & 31) && t >= col) {
+            if (which & 1) Q[t * kChunkLd + col] = sum[0];
+            else if (t > col) A[t * kChunkLd + col] = sum[0];
+        }
+    }
+    __syncthreads();
+    float* out = chunk_matrices(a, sd, blockIdx.z, blockIdx.y, h);
+    if (tid < kChunk) {  // column tid of T, by substitution
+        float x[kChunk];
+#pragma unroll
+        for (int t = 0; t < kChunk; ++t) {
+            float r = 0.f;
+#pragma unroll
+            for (int i = 0; i < t; ++i) r = fmaf(A[t * kChunkLd + i], x[i], r);
+            x[t] = (t == tid ? 1.f : 0.f) - coef[t].y * r;
+        }
+        const float beta = coef[tid].y;
+#pragma unroll
+        for (int t = 0; t < kChunk; ++t) out[t * kChunkLd + tid] = t >= tid ? x[t] * beta : 0.f;
+    } else if (tid >= 64) {
+        const int t = (tid - 64) >> 2, c = tid & 3;
+        *reinterpret_cast<float4*>(out + (kChunk + t) * kChunkLd + c * 4) = *reinterpret_cast<const float4*>(Q + t * kChunkLd + c * 4);
+    }
+}
+
+// The chain from chunk to chunk: a warp owns 32 / L * NC columns of one (sequence, head), L lanes 16 rows each of a group of NC of them
+// in registers, two warps per CTA share the chunks' rows (staged two deep by asynchronous copies).  Per chunk and column 48 D
+// multiply-adds against the state and about 272 among the tokens, each row read from shared memory meeting NC columns.  Bound by
+// the issue rate and the shared-memory reads of a warp or two per scheduler (ncu: 2.6 cycles per instruction, half of them the
+// two-cycle fma.f32x2).  Measured against the token-by-token form (one launch, 4 instead of 7 operations per state element but a
+// reduction and 1200 cycles per token): 8 x 1024 tokens, 12 heads of 64 x 128, decay per channel, 638 us -> 38 + 292; 3652 tokens, 25 heads
+// of 128 x 128, 661 us -> 62 + 514.
+__host__ __device__ constexpr int delta_warp_cols(int L, int NC) { return 32 / L * NC; }
+constexpr int kScanWarps = 2;
+// floats of a staged chunk: k, q, decays, v, T and Q, decays per token
+__host__ __device__ constexpr int delta_tile_floats(int L, int NC, bool CH) {
+    return kChunk * ((CH ? 3 : 2) * 16 * L + ((kScanWarps * delta_warp_cols(L, NC) + 3) & ~3)) + kChunkFloats + 2 * kChunk;
+}
+// floats of a warp's own: R (then U with its decays), U, S^T q, products of decays up to and behind a token
+__host__ __device__ constexpr int delta_warp_floats(int L, int NC) { return 3 * kChunk * (((delta_warp_cols(L, NC) + 3) & ~3) + 4) + 2 * kChunk; }
+
+template <int N> struct VecOf;
+template <> struct VecOf<1> { typedef float T; };
+template <> struct VecOf<2> { typedef float2 T; };
+template <> struct VecOf<4> { typedef float4 T; };
+template <int N>
+__device__ __forceinline__ void copy_vec(float* dst, const float* src) {
+    *reinterpret_cast<typename VecOf<N>::T*>(dst) = *reinterpret_cast<const typename VecOf<N>::T*>(src);
+}
+
+template <int L, int NC, bool CH>
+__global__ void __launch_bounds__(32 * kScanWarps)
+delta_scan_kernel(const DeltaArgs a) {
+    using Core = DeltaCore<L, NC, CH>;
+    using Row = typename Core::Row;
+    constexpr int D = 16 * L, VECS = CH ? 3 : 2, WC = delta_warp_cols(L, NC), COLS = kScanWarps * WC, THREADS = 32 * kScanWarps, CPAD = (COLS + 3) & ~3;
+    constexpr int WP = (WC + 3) & ~3, RS = WP + 4;     // a warp's columns in whole quads; row stride of its matrices
+    constexpr int TB = 16 / NC;                        // rows taken together against the state: 16 totals per group
+    constexpr int HELD = 16 / L, VW = HELD < NC ? HELD : NC;
+    constexpr int QUADS = WP / 4, TL = 32 / QUADS < kChunk ? 32 / QUADS : kChunk, NT = kChunk / TL;  // token x token products: a lane has a quad of columns, NT tokens
+    constexpr int TILE = delta_tile_floats(L, NC, CH);
+    extern __shared__ __align__(16) float sm[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* R = sm + 2 * TILE + D + warp * delta_warp_floats(L, NC);
+    float* U = R + kChunk * RS;
+    float* SQ = U + kChunk * RS;
+    float* upto = SQ + kChunk * RS;    // products of decays up to token t ...
+    float* behind = upto + kChunk;     // ... and of those behind it (one decay per head)
+    float* last = sm + 2 * TILE;       // CH: of the whole chunk, per dimension
+    const int h = blockIdx.x, c0 = blockIdx.y * COLS;
+    const int kvh = h / (a.H / a.G);
+    // rows of k and q beyond the head's dimension and columns beyond Dv stay zero in both tiles
+    for (int i = tid; i < 2 * TILE; i += THREADS) sm[i] = 0.f;
+    for (int i = lane; i < delta_warp_floats(L, NC); i += 32) R[i] = 0.f;
+    griddep_wait();
+    griddep_launch_dependents();
+    const SeqDesc sd = a.seqs[blockIdx.z];
+    const int grp = lane / L, l = lane & (L - 1);
+    const int wc = warp * WC, gc = wc + grp * NC;  // first column of the warp and of this group, in the CTA's
+    const int ncol = min(NC, a.Dv - c0 - gc);      // may be <= 0
     Core core;
-    float* Sg = a.S + (((size_t)sd.slot * a.H + h) * a.Dv + (gc < a.Dv ? gc : 0)) * D;
+    float* Sg = a.S + (((size_t)sd.slot * a.H + h) * a.Dv + (c0 + gc < a.Dv ? c0 + gc : 0)) * D;
     if (sd.pos0 > 0) core.load(Sg, l, ncol);
     else core.zero();
     __syncthreads();
 
-    const int d4 = a.Dl >> 2, v4 = min(cpad, a.Dvl - c0) >> 2;  // (c0 is a multiple of 4)
+    const int d4 = a.Dl >> 2, v4 = min(CPAD, a.Dvl - c0) >> 2;  // (c0 is a multiple of 4)
     const float* src0 = a.qkv + (size_t)sd.row0 * a.ld;
     auto stage = [&](int t0, int buf) {
-        float* q = sm + buf * tile_f;
-        const int nt = min(TOK, sd.n - t0);
+        float* k = sm + buf * TILE;
+        const int nt = min(kChunk, sd.n - t0);
         const int per = VECS * d4 + v4;
-        for (int j = tid; j < per; j += blockDim.x) {  // a 16-byte column piece of all tokens
+        for (int j = tid; j < per; j += THREADS) {  // a 16-byte column piece of all tokens
             const float* src = src0 + (size_t)t0 * a.ld;
             float* dst;
             int step = D, ld = a.ld;
-            if (j < d4) { src += kvh * a.Dl + j * 4; dst = q + j * 4; }
-            else if (j < 2 * d4) { src += a.k_col + kvh * a.Dl + (j - d4) * 4; dst = q + TOK * D + (j - d4) * 4; }
+            if (j < d4) { src += a.k_col + kvh * a.Dl + j * 4; dst = k + j * 4; }
+            else if (j < 2 * d4) { src += kvh * a.Dl + (j - d4) * 4; dst = k + kChunk * D + (j - d4) * 4; }
             else if (CH && j < 3 * d4) {
                 ld = a.ld_decay;
                 src = a.decay + (size_t)(sd.row0 + t0) * ld + (size_t)h * a.Dl + (j - 2 * d4) * 4;
-                dst = q + 2 * TOK * D + (j - 2 * d4) * 4;
-            } else { src += a.v_col + h * a.Dvl + c0 + (j - VECS * d4) * 4; dst = q + VECS * TOK * D + (j - VECS * d4) * 4; step = cpad; }
+                dst = k + 2 * kChunk * D + (j - 2 * d4) * 4;
+            } else { src += a.v_col + h * a.Dvl + c0 + (j - VECS * d4) * 4; dst = k + VECS * kChunk * D + (j - VECS * d4) * 4; step = CPAD; }
             for (int t = 0; t < nt; ++t) cp_async16(dst + t * step, src + (size_t)t * ld);
         }
-        if (tid < nt) cp_async16(q + TOK * (VECS * D + cpad) + tid * 4, a.coef + (size_t)(sd.row0 + t0 + tid) * a.H + h);
+        float* m = k + kChunk * (VECS * D + CPAD);
+        const float* msrc = chunk_matrices(a, sd, blockIdx.z, t0 / kChunk, h);
+        for (int i = tid; i < kChunkFloats / 4; i += THREADS) cp_async16(m + i * 4, msrc + i * 4);
+        if (!CH && tid < nt) cp_async8(m + kChunkFloats + tid * 2, a.coef + (size_t)(sd.row0 + t0 + tid) * a.H + h);
         cp_async_commit();
     };
     stage(0, 0);
-    const int oc = Core::ocol(lane);
-    const bool ow = Core::owns_o(lane);
-    float* orow = a.out + (size_t)sd.row0 * a.ldo + h * a.Dvl + gc + oc;
-    for (int t0 = 0, it = 0; t0 < sd.n; t0 += TOK, ++it) {
-        const int buf = it & 1, nt = min(TOK, sd.n - t0);
-        if (t0 + TOK < sd.n) { stage(t0 + TOK, buf ^ 1); cp_async_wait<1>(); }
+    const int quad = lane % QUADS, tlane = lane / QUADS;
+    const int oc = c0 + wc + quad * 4;  // this lane's quad of columns in the token x token products
+    const bool mine = tlane < TL && oc < a.Dv;
+    float* orow = a.out + (size_t)sd.row0 * a.ldo + h * a.Dvl + oc;
+    const int first = scatter_first<16, L>(lane);
+    for (int t0 = 0, it = 0; t0 < sd.n; t0 += kChunk, ++it) {
+        const int nt = min(kChunk, sd.n - t0);
+        if (t0 + kChunk < sd.n) { stage(t0 + kChunk, (it & 1) ^ 1); cp_async_wait<1>(); }
         else cp_async_wait<0>();
         __syncthreads();
-        const float* q = sm + buf * tile_f;
-        const float* k = q + TOK * D;
-        const float* gd = k + TOK * D;  // (CH)
-        const float* v = q + VECS * TOK * D + grp * NC;
-        const float* cf = q + TOK * (VECS * D + cpad);
-        typename Core::Row qr = Core::row(q, l), kr = Core::row(k, l), gr;
-        if (CH) gr = Core::row(gd, l);
-#pragma unroll 2
-        for (int t = 0; t < nt; ++t) {
-            const float4 co = *reinterpret_cast<const float4*>(cf + t * 4);
-            const int tn = min(t + 1, TOK - 1);
-            const typename Core::Row kn = Core::row(k + tn * D, l);
-            float o[Core::kOut];
-            core.token(kr, qr, q + tn * D, v + t * cpad, co.x, co.y, co.z, lane, o, &gr, gd + tn * D);
-            kr = kn;
-            if (ow) {
+        float* k = sm + (it & 1) * TILE;
+        float* q = k + kChunk * D;
+        float* kd = CH ? q + kChunk * D : k;  // the keys of the update (CH: over the decays)
+        const float* v = k + VECS * kChunk * D + wc;
+        const float* T = k + kChunk * (VECS * D + CPAD);
+        const float* Q = T + kChunk * kChunkLd;
+        float total = 1.f;
+        if (CH) {  // decays go into the rows: k and q those up to their token, kd those behind it
+            for (int d = tid; d < D; d += THREADS) {
+                float g[kChunk], kr[kChunk], p = 1.f;
 #pragma unroll
-                for (int j = 0; j < Core::kOut; ++j)
-                    if (oc + j < ncol) orow[j] = o[j];
+                for (int t = 0; t < kChunk; ++t) { g[t] = t < nt ? kd[t * D + d] : 1.f; kr[t] = k[t * D + d]; }
+#pragma unroll
+                for (int t = 0; t < kChunk; ++t) {
+                    p *= g[t];
+                    k[t * D + d] = kr[t] * p;
+                    q[t * D + d] *= p;
+                }
+                last[d] = p;
+                p = 1.f;
+#pragma unroll
+                for (int t = kChunk - 1; t >= 0; --t) {
+                    kd[t * D + d] = kr[t] * p;
+                    p *= g[t];
+                }
             }
-            orow += a.ldo;
+            __syncthreads();
+        } else {
+            const float g = lane < nt ? T[kChunkFloats + (lane & 15) * 2] : 1.f;
+            float up = g, down = g;
+#pragma unroll
+            for (int s = 1; s < kChunk; s <<= 1) {
+                const float x = __shfl_up_sync(0xffffffffu, up, s), y = __shfl_down_sync(0xffffffffu, down, s);
+                if (lane >= s) up *= x;
+                if (lane + s < kChunk) down *= y;
+            }
+            const float after = __shfl_down_sync(0xffffffffu, down, 1);
+            if (lane < kChunk) { upto[lane] = up; behind[lane] = lane + 1 < kChunk ? after : 1.f; }
+            total = __shfl_sync(0xffffffffu, up, kChunk - 1);
+            __syncwarp();
+        }
+        // S^T k and S^T q, TB rows at a time: 16 totals per group, spread over its lanes
+#pragma unroll 2
+        for (int r0 = 0; r0 < 2 * kChunk; r0 += TB) {
+            uint64_t acc[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[i] = 0ull;
+#pragma unroll
+            for (int r = 0; r < TB; ++r) {
+                const Row x = Core::row(k + (r0 + r) * D, l);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) acc[r * NC + j] = fma2(x.r[i], core.S[j][i], acc[r * NC + j]);
+            }
+            float tot[16];
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+                float x, y;
+                unpack2(acc[i], x, y);
+                tot[i] = x + y;
+            }
+            reduce_scatter<16, L>(tot, lane);
+#pragma unroll
+            for (int i = 0; i < HELD; i += VW) {
+                const int r = r0 + (first + i) / NC, col = grp * NC + (first + i) % NC;
+                float x[VW];
+                if (r0 < kChunk) {
+                    copy_vec<VW>(x, v + r * CPAD + col);
+                    const float p = CH ? 1.f : upto[r];
+#pragma unroll
+                    for (int e = 0; e < VW; ++e) x[e] -= p * tot[i + e];
+                    copy_vec<VW>(R + r * RS + col, x);
+                } else {
+                    const float p = CH ? 1.f : upto[r - kChunk];
+#pragma unroll
+                    for (int e = 0; e < VW; ++e) x[e] = p * tot[i + e];
+                    copy_vec<VW>(SQ + (r - kChunk) * RS + col, x);
+                }
+            }
+        }
+        __syncwarp();
+        // acc[i] += sum over j <= t of M[t, j] X[j, quad] for the tokens t = tlane + i * TL of this lane
+        uint64_t acc[NT][2];
+        auto below = [&](const float* M, const float* X) {
+#pragma unroll
+            for (int jb = 0; jb < kChunk; jb += 4) {
+                ulonglong2 x[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) x[j] = *reinterpret_cast<const ulonglong2*>(X + (jb + j) * RS + quad * 4);
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                    if (jb > i * TL + TL - 1) continue;
+                    const int t = (tlane + i * TL) & (kChunk - 1);
+                    const float4 m = *reinterpret_cast<const float4*>(M + t * kChunkLd + jb);
+                    const float mm[4] = {m.x, m.y, m.z, m.w};
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint64_t m2 = pack2(mm[j], mm[j]), lo = fma2(m2, x[j].x, acc[i][0]), hi = fma2(m2, x[j].y, acc[i][1]);
+                        if (jb + j <= i * TL || jb + j <= t) { acc[i][0] = lo; acc[i][1] = hi; }  // (a later token's row is not touched)
+                    }
+                }
+            }
+        };
+#pragma unroll
+        for (int i = 0; i < NT; ++i) acc[i][0] = acc[i][1] = 0ull;
+        below(T, R);
+        __syncwarp();  // R has been read
+        if (tlane < TL) {
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                const int t = tlane + i * TL;
+                *reinterpret_cast<ulonglong2*>(U + t * RS + quad * 4) = make_ulonglong2(acc[i][0], acc[i][1]);
+                if (!CH) {
+                    const uint64_t p = pack2(behind[t], behind[t]);
+                    *reinterpret_cast<ulonglong2*>(R + t * RS + quad * 4) = make_ulonglong2(mul2(p, acc[i][0]), mul2(p, acc[i][1]));
+                }
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(SQ + ((tlane + i * TL) & (kChunk - 1)) * RS + quad * 4);
+            acc[i][0] = x.x; acc[i][1] = x.y;
+        }
+        __syncwarp();
+        below(Q, U);
+        if (mine) {
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+                const int t = tlane + i * TL;
+                float o[4];
+                unpack2(acc[i][0], o[0], o[1]);
+                unpack2(acc[i][1], o[2], o[3]);
+                if (t >= nt) continue;
+                float* p = orow + (size_t)(t0 + t) * a.ldo;
+                if (WC % 4 == 0 && oc + 4 <= a.Dv) *reinterpret_cast<float4*>(p) = make_float4(o[0], o[1], o[2], o[3]);
+                else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (e < WC && oc + e < a.Dv) p[e] = o[e];
+                }
+            }
+        }
+        // the state over the chunk
+        if (CH) {
+            const Row g = Core::row(last, l);
+#pragma unroll
+            for (int j = 0; j < NC; ++j)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) core.S[j][i] = mul2(g.r[i], core.S[j][i]);
+        } else {
+            const uint64_t p = pack2(total, total);
+#pragma unroll
+            for (int j = 0; j < NC; ++j)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) core.S[j][i] = mul2(p, core.S[j][i]);
+        }
+        const float* Ud = (CH ? U : R) + grp * NC;
+#pragma unroll 4
+        for (int t = 0; t < nt; ++t) {
+            const Row x = Core::row(kd + t * D, l);
+            float u[NC];
+            copy_vec<NC>(u, Ud + t * RS);
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                const uint64_t uu = pack2(u[j], u[j]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) core.S[j][i] = fma2(x.r[i], uu, core.S[j][i]);
+            }
         }
         __syncthreads();
     }
@@ -818,43 +1107,37 @@ int launch_delta_step_one(b200_ctx* ctx, const DeltaArgs& a, int E) {
     return B200_OK;
 }
 
-template <int L, int NC, bool CH>
-int launch_delta_scan_one(b200_ctx* ctx, const DeltaArgs& a, int E) {
-    constexpr int D = 16 * L;
-    const int groups = (a.Dv + NC - 1) / NC;
-    // two warps per CTA (a block of columns starts at a multiple of four columns)
-    int threads = (groups * L + 31) & ~31;
-    if (threads > 64) threads = 64;
-    while (threads / L * NC % 4) threads += 32;
-    const int cols = threads / L * NC, cpad = (cols + 3) & ~3;
-    const size_t smem = (size_t)(2 * delta_tile_floats(D, cpad, CH) + D) * 4;
-    if (smem > 200 * 1024) return B200_ERR_LIMIT;
+// A state's 16 L rows take L lanes; of NC columns per group four read the least shared memory per multiply-add, two leave more warps to
+// hide the reduction over more lanes.  Measured (8 x 1024 tokens, 12 heads of 64 x 128, decay per channel): 292 us with four, 311 with
+// two, 446 with one; 3652 tokens, 25 heads of 128 x 128: 598, 514, 794.  Few sequences change nothing: 73, 73, 82 us for three of 37 to 250 tokens.
+template <int L, bool CH>
+int launch_delta_scan_ch(b200_ctx* ctx, const DeltaArgs& a, int E, int max_n) {
+    constexpr int NC = L >= 8 ? 2 : 4, D = 16 * L, cols = kScanWarps * delta_warp_cols(L, NC);
+    constexpr size_t rows = (size_t)(CH ? 3 : 2) * kChunk * (D + 4) * 4;
+    constexpr size_t need = (size_t)(2 * delta_tile_floats(L, NC, CH) + D + kScanWarps * delta_warp_floats(L, NC)) * 4, most = 226 * 1024;
+    static_assert(need <= most && cols % 4 == 0, "a CTA's columns");
+    // No more CTAs per SM than an even spread needs: they start while the kernel before them drains and would pile up where it ends
+    // first (shared memory that nobody uses keeps them apart; 292 and 359 us were seen for one launch of 192).
+    const dim3 grid(a.H, (a.Dv + cols - 1) / cols, E);
+    const size_t per_sm = ((size_t)grid.x * grid.y * grid.z + ctx->num_sms - 1) / ctx->num_sms;
+    const size_t smem = per_sm < 100 && most / per_sm - 1024 > need ? (most / per_sm - 1024) & ~(size_t)127 : need;
     static bool attr_set[64] = {};
     if (!attr_set[ctx->device & 63]) {
-        B200_CUDA(ctx, cudaFuncSetAttribute(delta_scan_kernel<L, NC, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        B200_CUDA(ctx, cudaFuncSetAttribute(delta_chunk_kernel<L, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows));
+        B200_CUDA(ctx, cudaFuncSetAttribute(delta_scan_kernel<L, NC, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
         attr_set[ctx->device & 63] = true;
     }
-    cudaError_t le = launch_pdl(ctx, delta_scan_kernel<L, NC, CH>, dim3(a.H, (a.Dv + cols - 1) / cols, E), dim3(threads), smem, a);
+    cudaError_t le = launch_pdl(ctx, delta_chunk_kernel<L, CH>, dim3(a.H, (max_n + kChunk - 1) / kChunk, E), dim3(128), rows, a);
+    ctx->launches++;
+    B200_CUDA(ctx, le);
+    le = launch_pdl(ctx, delta_scan_kernel<L, NC, CH>, grid, dim3(32 * kScanWarps), smem, a);
     ctx->launches++;
     B200_CUDA(ctx, le);
     return B200_OK;
 }
-
-// Columns per group: four are the cheapest per column, but with few sequences and heads the warps would be too
-// few to hide the chain from token to token.
-template <int L, bool CH>
-int launch_delta_scan_ch(b200_ctx* ctx, const DeltaArgs& a, int E) {
-    static const int forced = [] { const char* e = getenv("B200_DELTA_COLS"); return e ? atoi(e) : 0; }();  // tuning hook: 1, 2 or 4
-    const long columns = (long)a.H * E * a.Dv;
-    auto warps = [&](int nc) { return columns / nc * L / 32; };
-    const int nc = forced ? forced : (warps(4) >= 6L * ctx->num_sms ? 4 : (warps(2) >= 4L * ctx->num_sms ? 2 : 1));
-    if (nc == 4) return launch_delta_scan_one<L, 4, CH>(ctx, a, E);
-    if (nc == 2) return launch_delta_scan_one<L, 2, CH>(ctx, a, E);
-    return launch_delta_scan_one<L, 1, CH>(ctx, a, E);
-}
 template <int L>
-int launch_delta_scan_l(b200_ctx* ctx, const DeltaArgs& a, int E) {
-    return a.decay ? launch_delta_scan_ch<L, true>(ctx, a, E) : launch_delta_scan_ch<L, false>(ctx, a, E);
+int launch_delta_scan_l(b200_ctx* ctx, const DeltaArgs& a, int E, int max_n) {
+    return a.decay ? launch_delta_scan_ch<L, true>(ctx, a, E, max_n) : launch_delta_scan_ch<L, false>(ctx, a, E, max_n);
 }
 template <int L>
 int launch_delta_step_l(b200_ctx* ctx, const DeltaArgs& a, int E) {
@@ -897,6 +1180,8 @@ int launch_selective_scan(b200_ctx* ctx, const SelectiveScanArgs& a, int E, int 
     }
 }
 
+size_t delta_chunk_floats(int M, int E, int H) { return (size_t)((M + kChunk - 1) / kChunk + E) * H * kChunkFloats; }
+
 int delta_state_pad(int D) {
     for (int p = 32; p <= 256; p <<= 1)
         if (D <= p) return p;
@@ -927,12 +1212,12 @@ int launch_delta_prep(b200_ctx* ctx, const DeltaArgs& a, int E, int max_n) {
     return B200_OK;
 }
 
-int launch_delta_scan(b200_ctx* ctx, const DeltaArgs& a, int E) {
+int launch_delta_scan(b200_ctx* ctx, const DeltaArgs& a, int E, int max_n) {
     switch (delta_state_pad(a.D)) {
-        case 32: return launch_delta_scan_l<2>(ctx, a, E);
-        case 64: return launch_delta_scan_l<4>(ctx, a, E);
-        case 128: return launch_delta_scan_l<8>(ctx, a, E);
-        case 256: return launch_delta_scan_l<16>(ctx, a, E);
+        case 32: return launch_delta_scan_l<2>(ctx, a, E, max_n);
+        case 64: return launch_delta_scan_l<4>(ctx, a, E, max_n);
+        case 128: return launch_delta_scan_l<8>(ctx, a, E, max_n);
+        case 256: return launch_delta_scan_l<16>(ctx, a, E, max_n);
         default: return B200_ERR_LIMIT;
     }
 }

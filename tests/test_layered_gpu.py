@@ -427,3 +427,27 @@ def test_commands(pkg, tmp_path):
     r = subprocess.run([os.path.join(ROOT, "bin", "generate"), "--model", str(g), "--new", "6", "--prompt", "1,2,3"], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr
     assert len(r.stdout.strip().split(",")) == 6
+
+
+@pytest.mark.parametrize("dim,vdim", [(32, 40), (64, 128), (96, 28), (256, 20)])
+@pytest.mark.parametrize("channel", [False, True])
+def test_delta_rule_at_chunk_borders(pkg, ctx, dim, vdim, channel):
+    """The delta rule takes 16 tokens at a time: sequences that end before, at and behind a border, side by side and continued, in
+    32-bit arithmetic against float64 at the tolerance of the whole models."""
+    layer = delta(heads=2, kv_heads=1, dim=dim, vdim=vdim)
+    if channel:
+        layer["type"] = "channel_delta"
+    cfg = config([layer])
+    m, w = model(pkg, ctx, cfg, "float32", seed=3, max_slots=8)
+    lens = [1, 15, 16, 17, 31, 32, 33, 70]
+    toks = [tokens(cfg, n + 5, seed=n) for n in lens]
+    want = [L.forward(cfg, w, t) for t in toks]
+    slots = [m.open() for _ in lens]
+    for cut in (0, 1):  # prompts, then five more tokens each
+        parts = [t[n:] if cut else t[:n] for t, n in zip(toks, lens)]
+        got = m.step(list(zip(slots, parts)), want=np.arange(sum(map(len, parts))))
+        at = 0
+        for p, n, ref in zip(parts, lens, want):
+            check(got[at:at + len(p)], ref[n:] if cut else ref[:n], TOL["float32"], f"{n} {cut}")
+            at += len(p)
+    m.close()

@@ -40,8 +40,6 @@ struct b200_gpt2 {
     bool keep_kv = false;                        // the forward being enqueued also fills the cache
     int* pos_dev = nullptr;                      // position of the decode step being run
     float* resid2 = nullptr;                     // second residual buffer of the decode step [16][C]
-    float* att_partial = nullptr;                // decode attention: softmax states of the position splits
-    unsigned int* att_counters = nullptr;        // ... and their arrival counters (zero between launches)
     int* gen_tokens = nullptr;                   // greedy generation: prompt and continuation [max_B][max_T]
     cudaEvent_t host_done[2] = {nullptr, nullptr};  // forward_host_enqueue / _wait: results of a slot are on the host
     int* h_slot_status = nullptr;                // pinned: the device status word as seen behind each slot's work
@@ -744,8 +742,6 @@ int b200_gpt2_destroy(b200_gpt2* m) {
     for (auto& g : m->decode_graphs) cudaGraphExecDestroy(g.second);
     if (m->pos_dev) cudaFree(m->pos_dev);
     if (m->resid2) cudaFree(m->resid2);
-    if (m->att_partial) cudaFree(m->att_partial);
-    if (m->att_counters) cudaFree(m->att_counters);
     if (m->gen_tokens) cudaFree(m->gen_tokens);
     for (cudaEvent_t e : m->host_done) if (e) cudaEventDestroy(e);
     if (m->h_slot_status) cudaFreeHost(m->h_slot_status);
@@ -1042,9 +1038,6 @@ int b200_gpt2_enable_kv_cache(b200_gpt2* m) {
     cudaError_t e = cudaMalloc(&m->vcache, n * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&m->pos_dev, sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&m->resid2, (size_t)16 * m->cfg.channels * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&m->att_partial, (size_t)16 * m->cfg.num_heads * 8 * 66 * sizeof(float));  // up to 8 position splits
-    if (e == cudaSuccess) e = cudaMalloc(&m->att_counters, (size_t)16 * m->cfg.num_heads * sizeof(unsigned int));
-    if (e == cudaSuccess) e = cudaMemset(m->att_counters, 0, (size_t)16 * m->cfg.num_heads * sizeof(unsigned int));
     if (e == cudaSuccess) e = cudaMalloc(&m->gen_tokens, (size_t)m->max_B * m->max_T * sizeof(int));
     if (e != cudaSuccess) {
         cudaFree(m->kcache);
@@ -1089,9 +1082,11 @@ static int enqueue_decode(b200_gpt2* m, const int* tokens, int B) {
     float* ra = m->residual;
     float* rb = m->resid2;
     const bool fuse_ln = C <= 1664;
-    // narrow projections are computed in K slices by more CTAs; the prologue that consumes them adds the slices up
-    const int ks_att = fuse_ln ? skinny_gemm_k_splits(ctx, C, C) : 1;
-    const int ks_fc = fuse_ln ? skinny_gemm_k_splits(ctx, 4 * C, C) : 1;
+    // projections of long rows are computed in K slices; the prologue that consumes them adds the slices up
+    const int ks_att = fuse_ln ? skinny_gemm_k_splits(B, C) : 1;
+    const int ks_fc = fuse_ln ? skinny_gemm_k_splits(B, 4 * C) : 1;
+    // every product asks for the next one's weights
+    const size_t square = (size_t)C * C * 4;
     DSTEP(launch_decode_encoder(ctx, ra, tokens, P + off[0], P + off[1], m->pos_dev, B, C, Vp));
     const float* branch = nullptr;  // what the next layernorm adds to the residual first
     for (int l = 0; l < L; ++l) {
@@ -1099,8 +1094,9 @@ static int enqueue_decode(b200_gpt2* m, const int* tokens, int B) {
         const float* qkvb = P + off[5] + (size_t)l * 3 * C;
         const float *ln1w = P + off[2] + (size_t)l * C, *ln1b = P + off[3] + (size_t)l * C;
         const float *ln2w = P + off[8] + (size_t)l * C, *ln2b = P + off[9] + (size_t)l * C;
+        const float *attw = P + off[6] + (size_t)l * C * C, *fcw = P + off[10] + (size_t)l * 4 * C * C, *fcpw = P + off[12] + (size_t)l * 4 * C * C;
         if (fuse_ln) {
-            DSTEP(launch_skinny_gemm(ctx, m->qkv, ra, qkvw, qkvb, B, C, 3 * C, 0, branch, ln1w, ln1b, rb, 1, ks_fc));
+            DSTEP(launch_skinny_gemm(ctx, m->qkv, ra, qkvw, qkvb, B, C, 3 * C, 0, branch, ln1w, ln1b, rb, 1, ks_fc, attw, square));
             std::swap(ra, rb);
         } else {
             if (branch) {
@@ -1111,20 +1107,19 @@ static int enqueue_decode(b200_gpt2* m, const int* tokens, int B) {
             }
             DSTEP(launch_skinny_gemm(ctx, m->qkv, m->ln_out, qkvw, qkvb, B, C, 3 * C, 0));
         }
-        DSTEP(launch_decode_attention(ctx, m->atty, m->qkv, m->kcache + l * per_layer, m->vcache + l * per_layer, B, C, NH, m->pos_dev, m->max_T, m->att_partial, m->att_counters));
-        DSTEP(launch_skinny_gemm(ctx, m->branch, m->atty, P + off[6] + (size_t)l * C * C, P + off[7] + (size_t)l * C, B, C, C, 0,
-                                 nullptr, nullptr, nullptr, nullptr, ks_att));
-        const float* fcw = P + off[10] + (size_t)l * 4 * C * C;
+        DSTEP(launch_decode_attention(ctx, m->atty, m->qkv, m->kcache + l * per_layer, m->vcache + l * per_layer, B, C, NH, m->pos_dev, m->max_T));
+        DSTEP(launch_skinny_gemm(ctx, m->branch, m->atty, attw, P + off[7] + (size_t)l * C, B, C, C, 0,
+                                 nullptr, nullptr, nullptr, nullptr, ks_att, 1, fcw, 4 * square));
         const float* fcb = P + off[11] + (size_t)l * 4 * C;
         if (fuse_ln) {
-            DSTEP(launch_skinny_gemm(ctx, m->fch, ra, fcw, fcb, B, C, 4 * C, 1, m->branch, ln2w, ln2b, rb, 1, ks_att));
+            DSTEP(launch_skinny_gemm(ctx, m->fch, ra, fcw, fcb, B, C, 4 * C, 1, m->branch, ln2w, ln2b, rb, 1, ks_att, fcpw, 4 * square));
         } else {
             DSTEP(launch_fused_residual_layernorm(ctx, rb, m->ln_out, nullptr, nullptr, ra, m->branch, ln2w, ln2b, B, C, 0));
             DSTEP(launch_skinny_gemm(ctx, m->fch, m->ln_out, fcw, fcb, B, C, 4 * C, 1));
         }
         std::swap(ra, rb);
-        DSTEP(launch_skinny_gemm(ctx, m->branch, m->fch, P + off[12] + (size_t)l * C * 4 * C, P + off[13] + (size_t)l * C, B, 4 * C, C, 0,
-                                 nullptr, nullptr, nullptr, nullptr, ks_fc));
+        DSTEP(launch_skinny_gemm(ctx, m->branch, m->fch, fcpw, P + off[13] + (size_t)l * C, B, 4 * C, C, 0,
+                                 nullptr, nullptr, nullptr, nullptr, ks_fc, 1, l + 1 < L ? qkvw + (size_t)3 * C * C : nullptr, 3 * square));
         branch = m->branch;
     }
     // final layernorm and lm-head

@@ -130,18 +130,19 @@ int launch_attention_split(b200_ctx* ctx, float* out, float* lse, const uint16_t
 // k_splits > 1 (plain product only): K is cut into that many slices computed by different CTAs, and
 // out receives the partial results [k_splits][B][N] (the bias in slice 0) for a consumer that adds them
 // up in order - the layernorm prologue does, given branch_parts = the producer's k_splits
+// next: memory that a later kernel will read first (16-byte aligned), asked for into L2 while this one waits for its input
 int launch_skinny_gemm(b200_ctx* ctx, float* out, const float* x, const float* W, const float* bias, int B,
                        int K, int N, int gelu, const float* branch = nullptr, const float* ln_w = nullptr,
-                       const float* ln_b = nullptr, float* resid_out = nullptr, int k_splits = 1, int branch_parts = 1);
-int skinny_gemm_k_splits(const b200_ctx* ctx, int K, int N);  // the slices worth using for a [*,K] x [N,K]^T product
+                       const float* ln_b = nullptr, float* resid_out = nullptr, int k_splits = 1, int branch_parts = 1,
+                       const void* next = nullptr, size_t next_bytes = 0);
+int skinny_gemm_k_splits(int B, int K);  // the slices worth using for a product [B,K] x [N,K]^T
 // k and v columns of qkv rows [B*T, 3C] -> caches [B][cache_T][C] at positions pos0 .. pos0+T-1
 int launch_kv_append(b200_ctx* ctx, float* kcache, float* vcache, const float* qkv, int B, int T, int C, int pos0,
                      int cache_T);
 // out[B,C]: stores k and v of the rows qkv[B,3C] at position *pos_ptr, then attention of their
 // query parts over cached positions 0 .. *pos_ptr
-// partial: scratch of B * NH * 4 * 66 floats; counters: B * NH zeroed words (left zeroed)
 int launch_decode_attention(b200_ctx* ctx, float* out, const float* qkv, float* kcache, float* vcache, int B, int C,
-                            int NH, const int* pos_ptr, int cache_T, float* partial, unsigned int* counters);
+                            int NH, const int* pos_ptr, int cache_T);
 // out[B,C] = wte[tok[b]] + wpe[*pos_ptr]
 int launch_decode_encoder(b200_ctx* ctx, float* out, const int* tok, const float* wte, const float* wpe,
                           const int* pos_ptr, int B, int C, int vocab_rows);

@@ -38,8 +38,8 @@ int b200_get_tensor_map(b200_ctx* ctx, CUtensorMap* out, const float* ptr, uint6
 }
 
 int b200_get_tensor_map_bf16(b200_ctx* ctx, CUtensorMap* out, const void* ptr, uint64_t rows,
-                             uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols) {
-    TensorMapKey key{ptr, rows, cols, ld, box_rows, box_cols, 2};  // 2: 16-bit elements
+                             uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols, bool swizzle64) {
+    TensorMapKey key{ptr, rows, cols, ld, box_rows, box_cols, swizzle64 ? 4 : 2};  // 2: 16-bit elements; 4: the same, 64-byte swizzle
     auto it = ctx->tmap_cache.find(key);
     if (it != ctx->tmap_cache.end()) { *out = it->second; return B200_OK; }
     if (!ctx->encode_tiled) return B200_ERR_STATE;
@@ -50,7 +50,7 @@ int b200_get_tensor_map_bf16(b200_ctx* ctx, CUtensorMap* out, const void* ptr, u
     const cuuint32_t estr[2] = {1, 1};
     CUtensorMap m;
     CUresult r = ctx->encode_tiled(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims,
-                                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         ctx->last_error = "cuTensorMapEncodeTiled (bf16) failed with CUresult " + std::to_string((int)r);

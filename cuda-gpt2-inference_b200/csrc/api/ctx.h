@@ -70,9 +70,9 @@ int b200_get_tensor_map(b200_ctx* ctx, CUtensorMap* out, const float* ptr, uint6
                         uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols,
                         int swizzle_atom32 = 0);
 
-// The same over a matrix of bf16 (16-bit) elements: 128-byte swizzle of 16-byte chunks.
+// The same over a matrix of bf16 (16-bit) elements: 128-byte (64-byte) swizzle of 16-byte chunks.
 int b200_get_tensor_map_bf16(b200_ctx* ctx, CUtensorMap* out, const void* ptr, uint64_t rows,
-                             uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols);
+                             uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols, bool swizzle64 = false);
 
 // The same over a matrix of 8-bit elements (e4m3 operands of the fp8 GEMM).
 int b200_get_tensor_map_u8(b200_ctx* ctx, CUtensorMap* out, const void* ptr, uint64_t rows,

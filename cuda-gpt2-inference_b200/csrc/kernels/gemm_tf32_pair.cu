@@ -295,8 +295,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         // ---------------------------------------------------------------- epilogue
         const int q = warp & 3;
         const int ew = warp - 2;  // 0..7
-        // column split in units of one chunk (two for a bf16 output, whose stores take 64 columns)
-        const int unit = args.out_h ? 2 : 1;
+        // column split in units of one chunk (two for a single 16-bit output, whose stores take 64 columns)
+        const int unit = args.out_h && !args.out_planes ? 2 : 1;
         bool ok = true;
         int tile_iter = 0;
         TileWalk walk(args, pair, num_pairs);
@@ -529,9 +529,10 @@ int launch_gemm_pair(b200_ctx* ctx, float* out, const void* inp, const void* inp
         if (st != B200_OK) return st;
         maps[1] = maps[0]; maps[3] = maps[2];
     }
-    // the output in 32 x 32 boxes of fp32 (32 x 64 of bf16, both planes in one map), for the epilogue's TMA stores
+    // the output in 32 x 32 boxes of fp32 (32 x 64 of 16-bit values; 32 x 32 of two planes, both in one map), for the epilogue's TMA stores
     if (flags & (GEMM_GATED_GELU | GEMM_GATED_CLAMP)) maps[4] = maps[0];  // (not used: plain stores)
-    else if (out_h) st = b200_get_tensor_map_bf16(ctx, &maps[4], out_h, (uint64_t)M * (out_planes ? 2 : 1), (uint64_t)N, (uint64_t)N, 32, 64);
+    else if (out_planes) st = b200_get_tensor_map_bf16(ctx, &maps[4], out_h, (uint64_t)M * 2, (uint64_t)N, (uint64_t)N, 32, 32, true);
+    else if (out_h) st = b200_get_tensor_map_bf16(ctx, &maps[4], out_h, (uint64_t)M, (uint64_t)N, (uint64_t)N, 32, 64);
     else st = b200_get_tensor_map(ctx, &maps[4], out, (uint64_t)M, (uint64_t)N, (uint64_t)N, 32, 32);
     if (st != B200_OK) return st;
     // Tail of the tile sequence in narrow tiles (see GemmArgs::tail_sub): full-width tiles, whole in N, no K
